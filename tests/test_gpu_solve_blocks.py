@@ -52,3 +52,36 @@ def test_solve_repeated(gbx, cuda, N, NB, nrhs):
         X = B.clone()
         gbx.potrs_tiled(tiles, N, NB, X)
         assert _check(L, X, B)
+
+
+@pytest.mark.parametrize("NB", [65, 67, 95, 96, 97, 101, 113, 126, 127])
+@pytest.mark.parametrize("blocks", [0.4, 0.6, 1, 1.3, 2, 2.7, 9.9])
+def test_solve_tile_edges(gbx, cuda, NB, blocks):
+    """Tiles above 64 that no two equal blocks make up, and their neighbours: part of a tile, one, two and many of
+    them, the last one ragged."""
+    import torch
+    N = max(1, int(NB * blocks))
+    L, g = _factor(N, cuda, N + NB)
+    tiles = _tiles(gbx, L, NB)
+    for nrhs in (1, 3):
+        B = torch.randn(nrhs, N, dtype=torch.float64, device=cuda, generator=g)
+        X = B.clone()
+        gbx.potrs_tiled(tiles, N, NB, X)
+        assert _check(L, X, B)
+
+
+def test_solve_after_factor_odd_tile(gbx, cuda):
+    """Factorisation and solve of one system in tiles of 101: backward error of the whole call."""
+    import torch
+    N, NB = 707, 101
+    g = torch.Generator(device=cuda).manual_seed(3)
+    M = torch.rand(N, N, dtype=torch.float64, device=cuda, generator=g)
+    A = (M + M.T) / 2 - 0.5 + N * torch.eye(N, dtype=torch.float64, device=cuda)
+    tiles = _tiles(gbx, A.tril(), NB)
+    gbx.potrf_tiled(tiles, N, NB)
+    B = torch.randn(2, N, dtype=torch.float64, device=cuda, generator=g)
+    X = B.clone()
+    gbx.potrs_tiled(tiles, N, NB, X)
+    r = (A @ X.T).T - B
+    bound = 8 * N * np.finfo(np.float64).eps * (A.abs() @ X.abs().T).T
+    assert bool((r.abs() <= bound).all())
