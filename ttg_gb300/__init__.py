@@ -68,6 +68,7 @@ SIGNATURES = {
     "gbx_dgen_uniform_sym_tiled": (_i, [_i, _i, _ull, _d, _vp, _vp]),
     "gbx_dplgsy_tile": (_i, [_d, _i, _i, _vp, _i, _i, _i, _i, _ull, _vp]),
     "gbx_dag_timeout_selftest": (_i, [_i, _vp, _vp, _sz, _u64, _vp]),
+    "gbx_inv_timeout_selftest": (_i, [_i, _vp, _vp, _sz, _u64, _vp]),
     "gbx_dpotrf_tiled_noalloc": (_i, [_i, _i, _vp, _vp, _vp]),
     "gbx_gemm_bf16_nt_f32": (_i, [_i, _i, _i, _vp, _i, _vp, _i, _vp, _i, _vp, _vp]),
     "gbx_dgen_lowrank_sym_tiled": (_i, [_i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp]),
@@ -302,7 +303,9 @@ def split_f64(a, stream=None):
 
 
 def potri_tiled(tiles, N, NB, workspace=None, stream=None):
-    """In place: the lower tiles of the factor L (from potrf_tiled) become the lower triangle of A^{-1}."""
+    """In place: the lower tiles of the factor L (from potrf_tiled) become the lower triangle of A^{-1}.
+    Asynchronous. With gbx_set_fp64_update(1) a wait inside may run out: the triangle is NaN then, and
+    potrf_status(workspace) is GBX_ERR_TIMEOUT where the caller gave the workspace."""
     import torch
     need = _sz(0)
     call("gbx_dpotri_tiled_bufferSize", N, NB, ctypes.byref(need))

@@ -27,7 +27,8 @@
 namespace gbx {
 // potrf_f64.cu: the inverse as tasks of the tensor-core executor
 size_t inv_workspace_bytes(int N);
-int inv_run(int N, int NB, double* tiles, void* work, size_t work_bytes, cudaStream_t s);
+int inv_run(int N, int NB, double* tiles, void* work, size_t work_bytes, cudaStream_t s, long long first_task,
+            uint64_t timeout_ns);
 
 namespace potri {
 
@@ -274,7 +275,8 @@ extern "C" int gbx_dpotri_tiled(int N, int NB, double* tiles, void* work, size_t
   cudaStream_t s = (cudaStream_t)stream;
   // tensor-core updates where the caller has chosen them and the workspace holds their planes (one sized for
   // the FP64 form keeps that form)
-  if (gbx_get_fp64_update() == 1 && work_bytes >= inv_workspace_bytes(N)) return inv_run(N, NB, tiles, work, work_bytes, s);
+  if (gbx_get_fp64_update() == 1 && work_bytes >= inv_workspace_bytes(N))
+    return inv_run(N, NB, tiles, work, work_bytes, s, 0, gbx_get_wait_timeout_ns());
   static int attr_done = 0;  // benign race: every caller sets the same value
   if (!attr_done) {
     if (cudaFuncSetAttribute(diag_inverse64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -326,5 +328,7 @@ extern "C" int gbx_dpotri_tiled(int N, int NB, double* tiles, void* work, size_t
     if (int e = launch_step<LAUUM_DIAG>(a, 1, s)) return e;
     copy_tiles_kernel<<<64, 256, 0, s>>>(S, T(k, k), tl, NB, 1);
   }
+  // no wait in this form can run out; S, which held the status word's bytes, is not needed any more
+  if (cudaMemsetAsync(work, 0, sizeof(DagState), s) != cudaSuccess) return GBX_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? GBX_OK : GBX_ERR_CUDA;
 }
