@@ -2,7 +2,7 @@
 // launch (no host round trip, capturable in a CUDA graph).
 //
 // Each CTA takes matrices from a device-side queue in the order the caller gives (largest first is
-// the longest-processing-time schedule) and for each matrix runs, on 128 threads:
+// the longest-processing-time schedule) and for each matrix runs, on 128 or 256 threads:
 //   plain (FP64):  left-looking Cholesky by 64 x 64 blocks, then the forward/backward solve for its
 //                  right-hand sides, all in place;
 //   fp32 + IR:     an FP32 factor of the same form, FP32 solve, then `refine` steps of FP64 iterative
@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <numeric>
 #include <type_traits>
@@ -28,11 +29,10 @@ namespace batched {
 
 constexpr int kMaxN = 1024;  // largest matrix order of the batched kernel (shared-memory vectors)
 // One matrix keeps one CTA busy in spurts (a chain of pivots, a block product, a chain of panel solves), so
-// a CTA is small and four matrices share an SM. 4096 matrices of 32 .. 512 rows: FP64 90.2 -> 56.3 ms with one CTA of
-// 256 threads per SM before (the FP64 pipe alone needs 46), FP32 and two refinements 14.4 -> 8.9 (two CTAs of 256).
-constexpr int kThr = 128, kWarps = kThr / 32;
-constexpr int kPan = 64;            // block edge of the factorisation
-constexpr int kCols = kPan / kWarps;  // columns of a block per warp
+// a CTA is small and four matrices share an SM; two with twice the warps when there are few (gbx_dposv_batched_ex).
+// 4096 matrices of 32 .. 512 rows: FP64 90.2 -> 55.7 ms with one CTA of 256 threads per SM before (the FP64 pipe alone
+// needs 46), FP32 and two refinements 14.4 -> 8.9 (two CTAs of 256).
+constexpr int kPan = 64;            // largest block edge of the factorisation
 constexpr int kCk = 8;              // k-chunk of the block products
 // shared memory of the FP64 factorisation: the panel's triangle, two chunks of both operands, the last columns, one int
 constexpr size_t kFactor64Smem = (size_t)(kPan * kPan + 4 * kCk * kPan + 256) * sizeof(double) + 16;
@@ -45,9 +45,14 @@ constexpr size_t kFactor64Smem = (size_t)(kPan * kPan + 4 * kCk * kPan + 256) * 
 
 // u += L(r0.., 0:p0) L(p0.., 0:p0)^T; mb, pb: rows and columns present. k in chunks through shared memory, the next
 // chunk in registers; a thread's columns stand in a row in the second operand.
-__device__ __forceinline__ void panel_update(double (&u)[2][kCols], const double* L, int ld, int r0, int p0, int mb, int pb, double* sm) {
+// NG: groups of 16 columns; kLow: rows 32.. exist; kDiag: a diagonal block, whose first 32 rows have no columns past 32.
+// (Parameters of the loop, since an FP64 instruction that a predicate turns off takes its time on the pipe all the same.)
+template <int W, int NG, bool kLow, bool kDiag>
+__device__ __forceinline__ void panel_update(double (&u)[2][kPan / W], const double* L, int ld, int r0, int p0, int mb, int pb,
+                                             double* sm) {
   using T = double;
-  constexpr int CK = kCk, NL = CK * kPan / kThr;  // loads per thread, chunk and operand
+  constexpr int kWarps = W, kThr = 32 * W, kCols = kPan / W;
+  constexpr int CK = kCk, NL = CK * kPan / kThr, KS = kThr / kPan;  // loads per thread, chunk and operand; their step in k
   T* As = sm;                 // [2][CK][64]
   T* Bs = sm + 2 * CK * kPan;  // [2][CK][64], column c at (c % kWarps) kCols + c / kWarps
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = tid & 63, kk = tid >> 6;
@@ -58,7 +63,7 @@ __device__ __forceinline__ void panel_update(double (&u)[2][kCols], const double
   auto load = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < NL; ++i) {
-      const long long k = (long long)(k0 + kk + 2 * i) * ld;  // p0 is a multiple of 64: whole chunks
+      const long long k = (long long)(k0 + kk + KS * i) * ld;  // p0 is a multiple of 64: whole chunks
       va[i] = Ap[k];
       vb[i] = Bp[k];
     }
@@ -66,11 +71,10 @@ __device__ __forceinline__ void panel_update(double (&u)[2][kCols], const double
   auto store = [&](int buf) {
 #pragma unroll
     for (int i = 0; i < NL; ++i) {
-      As[(buf * CK + kk + 2 * i) * kPan + row] = va[i];
-      Bs[(buf * CK + kk + 2 * i) * kPan + at] = vb[i];
+      As[(buf * CK + kk + KS * i) * kPan + row] = va[i];
+      Bs[(buf * CK + kk + KS * i) * kPan + at] = vb[i];
     }
   };
-  const bool low = mb > 32;
   load(0);
   store(0);
   __syncthreads();
@@ -79,18 +83,20 @@ __device__ __forceinline__ void panel_update(double (&u)[2][kCols], const double
 #pragma unroll
     for (int k = 0; k < CK; ++k) {
       const T* ar = As + (buf * CK + k) * kPan + lane;
-      const T a0 = ar[0], a1 = ar[32];
+      const T* br = Bs + (buf * CK + k) * kPan + kCols * warp;
+      const T a0 = ar[0], a1 = kLow ? ar[32] : T(0);
 #pragma unroll
-      for (int q = 0; q < kCols; q += 4)
-        if (kWarps * q < pb) {  // (uniform)
-          T b[4];
-          lds4(Bs + (buf * CK + k) * kPan + kCols * warp + q, b);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            u[0][q + e] = fma(a0, b[e], u[0][q + e]);
-            if (low) u[1][q + e] = fma(a1, b[e], u[1][q + e]);
-          }
+      for (int e = 0; e < NG * 16 / W; e += 2) {
+        const double2 b = *(const double2*)(br + e);
+        if (!kDiag || kWarps * e < 32) {
+          u[0][e] = fma(a0, b.x, u[0][e]);
+          u[0][e + 1] = fma(a0, b.y, u[0][e + 1]);
         }
+        if (kLow) {
+          u[1][e] = fma(a1, b.x, u[1][e]);
+          u[1][e + 1] = fma(a1, b.y, u[1][e + 1]);
+        }
+      }
     }
     if (k0 + CK < p0) store(buf ^ 1);
     __syncthreads();
@@ -98,8 +104,9 @@ __device__ __forceinline__ void panel_update(double (&u)[2][kCols], const double
 }
 
 // The block's columns in turn: for q, jj (column j = kWarps q + jj < n, owned by warp jj) f(q, jj) with q a constant
-template <typename F>
+template <int W, typename F>
 __device__ __forceinline__ void each_column(int n, F f) {
+  constexpr int kWarps = W, kCols = kPan / W;
   auto round = [&](auto qc) {
     constexpr int q = decltype(qc)::value;
 #pragma unroll 1
@@ -108,17 +115,19 @@ __device__ __forceinline__ void each_column(int n, F f) {
     return true;
   };
 #define GBX_R(Q) if (!round(std::integral_constant<int, Q>{})) return;
-  static_assert(kCols == 16, "rounds");
+  static_assert(kCols == 16 || kCols == 8, "rounds");
   GBX_R(0) GBX_R(1) GBX_R(2) GBX_R(3) GBX_R(4) GBX_R(5) GBX_R(6) GBX_R(7)
-  GBX_R(8) GBX_R(9) GBX_R(10) GBX_R(11) GBX_R(12) GBX_R(13) GBX_R(14) GBX_R(15)
+  if constexpr (kCols == 16) { GBX_R(8) GBX_R(9) GBX_R(10) GBX_R(11) GBX_R(12) GBX_R(13) GBX_R(14) GBX_R(15) }
 #undef GBX_R
 }
 
 // Cholesky of the n x n diagonal block A - u, in place and, its columns divided by the diagonal, into tri. One barrier a column; the warp that owns the next pivot takes it before anything
 // else and applies the current column to its others together with its own (as chol64_regs). cb: three columns, then
 // the pivots' reciprocals. Returns 0 or the 1-based index of the first bad pivot.
-__device__ __forceinline__ int chol_block(double (&u)[2][kCols], double* A, int ld, int n, double* tri, double* cb, int* flag) {
+template <int W>
+__device__ __forceinline__ int chol_block(double (&u)[2][kPan / W], double* A, int ld, int n, double* tri, double* cb, int* flag) {
   using T = double;
+  constexpr int kWarps = W, kCols = kPan / W;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool low = n > 32;  // rows 32.. exist
   T a[2];
@@ -154,7 +163,7 @@ __device__ __forceinline__ int chol_block(double (&u)[2][kCols], double* A, int 
   if (warp < n) fetch(warp);
   if (warp == 0) pivot(std::integral_constant<int, 0>{}, 0);
   __syncthreads();
-  each_column(n, [&](auto qc, int jj) {
+  each_column<W>(n, [&](auto qc, int jj) {
     constexpr int q = decltype(qc)::value;
     const int j = kWarps * q + jj;
     const int f = *(volatile int*)flag;  // (a later pivot's failure waits for its own turn)
@@ -196,9 +205,11 @@ __device__ __forceinline__ int chol_block(double (&u)[2][kCols], double* A, int 
 }
 
 // A(mb rows, n columns) := (A - u) L11^{-T} against the triangle of chol_block; xb: 128 elements
-__device__ __forceinline__ void solve_block(double (&u)[2][kCols], double* A, int ld, int mb, int n, const double* tri,
+template <int W>
+__device__ __forceinline__ void solve_block(double (&u)[2][kPan / W], double* A, int ld, int mb, int n, const double* tri,
                                             const double* rinv, double* xb) {
   using T = double;
+  constexpr int kWarps = W, kCols = kPan / W;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool low = mb > 32;
   T a[2];
@@ -219,7 +230,7 @@ __device__ __forceinline__ void solve_block(double (&u)[2][kCols], double* A, in
   if (warp < n) fetch(warp);
   if (warp == 0) finish(std::integral_constant<int, 0>{}, 0);
   __syncthreads();
-  each_column(n, [&](auto qc, int jj) {
+  each_column<W>(n, [&](auto qc, int jj) {
     constexpr int q = decltype(qc)::value;
     const int j = kWarps * q + jj;
     const T* b = xb + 64 * (j & 1);
@@ -252,7 +263,9 @@ __device__ __forceinline__ void solve_block(double (&u)[2][kCols], double* A, in
 
 // FP64 left-looking Cholesky of an n x n column-major matrix (ld), in place, by 64 x 64 blocks: bound by the FP64 pipe.
 // Returns 0 or the 1-based index of the first bad pivot.
+template <int W>
 __device__ __forceinline__ int factor64(double* A, int n, int ld, unsigned char* smem) {
+  constexpr int kCols = kPan / W;
   double* tri = (double*)smem;
   double* cb = tri + kPan * kPan;
   double* stage = cb + 256;
@@ -266,13 +279,24 @@ __device__ __forceinline__ int factor64(double* A, int n, int ld, unsigned char*
       double u[2][kCols];
 #pragma unroll
       for (int q = 0; q < kCols; ++q) u[0][q] = u[1][q] = 0.0;
-      if (p0 > 0) panel_update(u, A, ld, r0, p0, mb, pb, stage);
+      if (p0 > 0) {
+        if (r0 == p0) {  // the last one may be narrow
+          if (pb <= 16) panel_update<W, 1, false, true>(u, A, ld, r0, p0, mb, pb, stage);
+          else if (pb <= 32) panel_update<W, 2, false, true>(u, A, ld, r0, p0, mb, pb, stage);
+          else if (pb <= 48) panel_update<W, 3, true, true>(u, A, ld, r0, p0, mb, pb, stage);
+          else panel_update<W, 4, true, true>(u, A, ld, r0, p0, mb, pb, stage);
+        } else if (mb <= 32) {
+          panel_update<W, 4, false, false>(u, A, ld, r0, p0, mb, pb, stage);
+        } else {
+          panel_update<W, 4, true, false>(u, A, ld, r0, p0, mb, pb, stage);
+        }
+      }
       double* o = A + r0 + (long long)p0 * ld;
       if (r0 == p0) {
-        const int info = chol_block(u, o, ld, pb, tri, cb, flag);
+        const int info = chol_block<W>(u, o, ld, pb, tri, cb, flag);
         if (info) return p0 + info;
       } else {
-        solve_block(u, o, ld, mb, pb, tri, cb + 192, cb);
+        solve_block<W>(u, o, ld, mb, pb, tri, cb + 192, cb);
       }
       __syncthreads();
     }
@@ -291,21 +315,21 @@ constexpr size_t kFactor32Smem = (size_t)(kPan * kLdS + 2 * kCk32 * kPan + kPan)
 // u[c] += sum over k < kd of L(row, k) L(brow + c, k), NC columns of the block at brow (pb of its rows present): the
 // second operand through shared memory in chunks of kCk32, the next chunk and the thread's own values in registers.
 // live: the warp has rows (else it only stages)
-template <int NC>
+template <int W, int NC>
 __device__ __forceinline__ void row_update(float (&u)[NC], const float* L, int ld, int row, int brow, int pb, int kd, int c0,
                                            bool live, float* Bs) {
   const int tid = threadIdx.x, bc = tid & 63, bk = tid >> 6;
   const float* Lr = L + row;
   const float* Lb = L + brow + (bc < pb ? bc : 0);
-  constexpr int NB = kCk32 * kPan / kThr;
+  constexpr int KS = 32 * W / kPan, NB = kCk32 / KS;  // step in k of a thread's loads, their number
   float a[kCk32], vb[NB];
   auto load = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < NB; ++i) vb[i] = Lb[(long long)(k0 + bk + 2 * i) * ld];
+    for (int i = 0; i < NB; ++i) vb[i] = Lb[(long long)(k0 + bk + KS * i) * ld];
   };
   auto store = [&](int buf) {
 #pragma unroll
-    for (int i = 0; i < NB; ++i) Bs[(buf * kCk32 + bk + 2 * i) * kPan + bc] = vb[i];
+    for (int i = 0; i < NB; ++i) Bs[(buf * kCk32 + bk + KS * i) * kPan + bc] = vb[i];
   };
   load(0);
   store(0);
@@ -337,7 +361,9 @@ __device__ __forceinline__ void row_update(float (&u)[NC], const float* L, int l
 
 // FP32 left-looking Cholesky by 64-column panels: the lower triangle of A, converted as it is read, into L.
 // As in FP64 the products are summed up by themselves and subtracted from A once.
+template <int W>
 __device__ __noinline__ int factor32(const double* A, float* L, int n, int ld, unsigned char* smem) {
+  constexpr int kThr = 32 * W;
   float* S = (float*)smem;          // the panel's triangle, column c at c kLdS
   float* Bs = S + kPan * kLdS;      // [2][kCk32][64]
   float* rinv = Bs + 2 * kCk32 * kPan;
@@ -345,14 +371,15 @@ __device__ __noinline__ int factor32(const double* A, float* L, int n, int ld, u
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int p0 = 0; p0 < n; p0 += kPan) {
     const int pb = min(kPan, n - p0);
-    {  // the diagonal block: thread = row (tid & 63), 32 columns
-      const int r = tid & 63, c0 = 32 * (tid >> 6), row = p0 + min(r, pb - 1);
-      float u[32];
+    {  // the diagonal block: thread = row (tid & 63), NC columns
+      constexpr int NC = kPan * kPan / kThr;
+      const int r = tid & 63, c0 = NC * (tid >> 6), row = p0 + min(r, pb - 1);
+      float u[NC];
 #pragma unroll
-      for (int c = 0; c < 32; ++c) u[c] = 0.f;
-      if (p0 > 0) row_update<32>(u, L, ld, row, p0, pb, p0, c0, true, Bs);
+      for (int c = 0; c < NC; ++c) u[c] = 0.f;
+      if (p0 > 0) row_update<W, NC>(u, L, ld, row, p0, pb, p0, c0, true, Bs);
 #pragma unroll
-      for (int c = 0; c < 32; ++c)
+      for (int c = 0; c < NC; ++c)
         if (r < pb && c0 + c <= r) S[(c0 + c) * kLdS + r] = (float)A[row + (long long)(p0 + c0 + c) * ld] - u[c];
     }
     __syncthreads();
@@ -379,24 +406,24 @@ __device__ __noinline__ int factor32(const double* A, float* L, int n, int ld, u
       }
       __syncthreads();
       {
-        float acc[8];
+        constexpr int NE = 32 / W;  // columns per warp
+        float acc[NE];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+        for (int e = 0; e < NE; ++e) acc[e] = 0.f;
 #pragma unroll 8
         for (int k = 0; k < 32; ++k) {
           const float a = S[k * kLdS + 32 + lane];
-          float b0[4], b1[4];
-          lds4(S + k * kLdS + 32 + 8 * warp, b0);
-          lds4(S + k * kLdS + 32 + 8 * warp + 4, b1);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[e] = fmaf(a, b0[e], acc[e]);
-            acc[4 + e] = fmaf(a, b1[e], acc[4 + e]);
+          for (int q = 0; q < NE; q += 4) {
+            float b[4];
+            lds4(S + k * kLdS + 32 + NE * warp + q, b);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[q + e] = fmaf(a, b[e], acc[q + e]);
           }
         }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int c = 8 * warp + e;
+        for (int e = 0; e < NE; ++e) {
+          const int c = NE * warp + e;
           if (lane < w2 && c <= lane) S[(32 + c) * kLdS + 32 + lane] -= acc[e];
         }
       }
@@ -412,14 +439,14 @@ __device__ __noinline__ int factor32(const double* A, float* L, int n, int ld, u
       const int r = e & 63, c = e >> 6;
       if (r < pb && c <= r) L[p0 + r + (long long)(p0 + c) * ld] = S[c * kLdS + r];
     }
-    // the rows below, 128 at a time (there are some only below a whole panel)
+    // the rows below, a thread each (there are some only below a whole panel)
     for (int r0 = p0 + kPan; r0 < n; r0 += kThr) {
       const bool live = r0 + 32 * warp < n;
       const int row = min(r0 + tid, n - 1);
       float u[kPan];
 #pragma unroll
       for (int c = 0; c < kPan; ++c) u[c] = 0.f;
-      if (p0 > 0) row_update<kPan>(u, L, ld, row, p0, kPan, p0, 0, live, Bs);
+      if (p0 > 0) row_update<W, kPan>(u, L, ld, row, p0, kPan, p0, 0, live, Bs);
       if (live) {
         const double* Ar = A + row + (long long)p0 * ld;
         float* Lr = L + row + (long long)p0 * ld;
@@ -451,8 +478,9 @@ __device__ __noinline__ int factor32(const double* A, float* L, int n, int ld, u
 // (L L^T)^{-1} on R right-hand sides in shared memory (xs[r * ldx + i]) at once, by panels of 32: warp r solves
 // the panel's triangle for right-hand side r; a thread applies it to its rows (forward), or a warp gathers the
 // solved rows below for its columns (backward). tri: 2 * 32 * 33 elements.
-template <typename T, int R>
+template <int W, typename T, int R>
 __device__ __forceinline__ void solve_multi(const T* L, int n, int ld, T* xs, int ldx, T* tri) {
+  constexpr int kWarps = W, kThr = 32 * W;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto load_tri = [&](int p0, T* t) {  // zeros outside the triangle and past n
 #pragma unroll
@@ -559,9 +587,9 @@ __device__ __forceinline__ void solve_multi(const T* L, int n, int ld, T* xs, in
 // xf = (float)(b - A x) for R right-hand sides, A symmetric from its lower triangle, everything in FP64: one thread per
 // row. (Past the diagonal a thread reads its own column of A, sixteen entries a cache line: bound by the FP64
 // pipe all the same. Reading those coalesced and adding up across lanes took twice as long.)
-template <int R>
+template <int W, int R>
 __device__ __forceinline__ void residual(const double* A, int n, const double* b, const double* xd, float* xf, int ldx) {
-  for (int i = threadIdx.x; i < n; i += kThr) {
+  for (int i = threadIdx.x; i < n; i += 32 * W) {
     double s[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) s[r] = b[i + (long long)r * n];
@@ -597,17 +625,19 @@ struct Params {
   int nrhs;
   int refine;    // IR steps
   int* info;     // per matrix: 0 or first bad pivot
-  unsigned long long* head;
+  unsigned long long* head;  // matrices taken from the front of the order (low half) and its end (high half) after the first
+  int front;                 // CTAs that take from the front
+  int sms;
 };
 
 // R right-hand sides b (column-major, n x R) of one factorised matrix, in place
-template <int MODE, int R>
+template <int MODE, int W, int R>
 __device__ __noinline__ void solve_rhs(const double* A, const float* L32, double* b, int n, int refine,
                                           unsigned char* smem) {
   const int ldx = (n + 3) & ~3;  // 16-byte rows
   const int tid = threadIdx.x;
   auto each = [&](auto f) {
-    for (int e = tid; e < n; e += kThr)
+    for (int e = tid; e < n; e += 32 * W)
 #pragma unroll
       for (int r = 0; r < R; ++r) f(r * ldx + e, e + (long long)r * n);
     __syncthreads();
@@ -616,17 +646,17 @@ __device__ __noinline__ void solve_rhs(const double* A, const float* L32, double
   if constexpr (MODE == 0) {
     double* tri = xd + R * ldx;
     each([&](int i, long long g) { xd[i] = b[g]; });
-    solve_multi<double, R>(A, n, n, xd, ldx, tri);
+    solve_multi<W, double, R>(A, n, n, xd, ldx, tri);
     each([&](int i, long long g) { b[g] = xd[i]; });
   } else {
     float* xf = (float*)(xd + R * ldx);
     float* tri = xf + R * ldx;
     each([&](int i, long long g) { xf[i] = (float)b[g]; });
-    solve_multi<float, R>(L32, n, n, xf, ldx, tri);
+    solve_multi<W, float, R>(L32, n, n, xf, ldx, tri);
     each([&](int i, long long) { xd[i] = (double)xf[i]; });
     for (int it = 0; it < refine; ++it) {
-      residual<R>(A, n, b, xd, xf, ldx);
-      solve_multi<float, R>(L32, n, n, xf, ldx, tri);
+      residual<W, R>(A, n, b, xd, xf, ldx);
+      solve_multi<W, float, R>(L32, n, n, xf, ldx, tri);
       each([&](int i, long long) { xd[i] += (double)xf[i]; });
     }
     each([&](int i, long long g) { b[g] = xd[i]; });
@@ -638,19 +668,33 @@ constexpr size_t solve_smem(int mode) {
 }
 constexpr size_t kSmem64 = std::max(kFactor64Smem, solve_smem(0));
 constexpr size_t kSmem32 = std::max(kFactor32Smem, solve_smem(1));
-constexpr int kCtas64 = 4, kCtas32 = 4;  // CTAs per SM: 128 registers; FP64 50 KB of shared memory, FP32 33 KB
+// CTAs per SM, of four and of eight warps: 128 registers; FP64 50 KB of shared memory, FP32 33 KB
+constexpr int ctas_per_sm(int W) { return 16 / W; }
 
-// MODE 0: plain FP64; MODE 1: fp32 + IR
-template <int MODE>
-__global__ void __launch_bounds__(kThr, MODE == 0 ? kCtas64 : kCtas32) batched_kernel(Params P) {
+// MODE 0: plain FP64; MODE 1: fp32 + IR; W: warps of a CTA
+template <int MODE, int W>
+__global__ void __launch_bounds__(32 * W, ctas_per_sm(W)) batched_kernel(Params P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_idx;
+  // The first matrix is the CTA's own, so that it is known which ones share an SM (CTAs go to the SMs in turn, and they all
+  // start at about the same time): every second round of SMs in reverse, and from the end of the order the other way round
+  // than from its front. Then what is left, from the CTA's end.
+  const int wave = (int)blockIdx.x / P.sms, in_wave = min(P.sms, P.front - wave * P.sms), at = (int)blockIdx.x % P.sms;
+  int first = (int)blockIdx.x >= P.front ? P.batch - 1 - ((int)blockIdx.x - P.front)
+                                         : wave * P.sms + (wave & 1 ? in_wave - 1 - at : at);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      const unsigned long long t = atomicAdd(P.head, 1ULL);
-      s_idx = t < (unsigned long long)P.batch ? P.order[t] : -1;
+      long long t = first;
+      if (first < 0) {
+        const bool front = (int)blockIdx.x < P.front;
+        const unsigned long long h = atomicAdd(P.head, front ? 1ULL : 1ULL << 32);
+        const long long f = P.front + (long long)(h & 0xffffffffULL), e = gridDim.x - P.front + (long long)(h >> 32);
+        t = f + e >= P.batch ? -1 : front ? f : P.batch - 1 - e;  // (f and e of them are taken)
+      }
+      s_idx = t >= 0 ? P.order[t] : -1;
     }
+    first = -1;
     __syncthreads();
     const int idx = s_idx;
     if (idx < 0) break;
@@ -662,8 +706,8 @@ __global__ void __launch_bounds__(kThr, MODE == 0 ? kCtas64 : kCtas32) batched_k
       }
       double* A = P.A + P.offA[idx];
       int inf;
-      if constexpr (MODE == 0) inf = factor64(A, n, n, smem_raw);
-      else inf = factor32(A, P.L32 + P.offA[idx], n, n, smem_raw);
+      if constexpr (MODE == 0) inf = factor64<W>(A, n, n, smem_raw);
+      else inf = factor32<W>(A, P.L32 + P.offA[idx], n, n, smem_raw);
       __syncthreads();
       if (threadIdx.x == 0) P.info[idx] = inf;
       if (inf) continue;
@@ -678,16 +722,16 @@ __global__ void __launch_bounds__(kThr, MODE == 0 ? kCtas64 : kCtas32) batched_k
       double* b = B + (long long)j * n;
       const int left = P.nrhs - j;
       if (most == 4 && left >= 4) {
-        solve_rhs<MODE, 4>(A, L, b, n, P.refine, smem_raw);
+        solve_rhs<MODE, W, 4>(A, L, b, n, P.refine, smem_raw);
         j += 4;
       } else if (most == 4 && left == 3) {
-        solve_rhs<MODE, 3>(A, L, b, n, P.refine, smem_raw);
+        solve_rhs<MODE, W, 3>(A, L, b, n, P.refine, smem_raw);
         j += 3;
       } else if (left >= 2) {
-        solve_rhs<MODE, 2>(A, L, b, n, P.refine, smem_raw);
+        solve_rhs<MODE, W, 2>(A, L, b, n, P.refine, smem_raw);
         j += 2;
       } else {
-        solve_rhs<MODE, 1>(A, L, b, n, P.refine, smem_raw);
+        solve_rhs<MODE, W, 1>(A, L, b, n, P.refine, smem_raw);
         ++j;
       }
     }
@@ -697,6 +741,10 @@ __global__ void __launch_bounds__(kThr, MODE == 0 ? kCtas64 : kCtas32) batched_k
 std::mutex g_mtx;
 int g_sms = 0;
 bool g_attr = false;
+template <int MODE, int W>
+int set_smem(size_t bytes) {
+  return cudaFuncSetAttribute(batched_kernel<MODE, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess;
+}
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   z += 0x9e3779b97f4a7c15ULL;
@@ -773,10 +821,7 @@ extern "C" int gbx_dposv_batched_ex(int batch, const int* n, const long long* of
       int dev = 0;
       cudaGetDevice(&dev);
       if (cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return GBX_ERR_CUDA;
-      if (cudaFuncSetAttribute(batched_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem64) !=
-              cudaSuccess ||
-          cudaFuncSetAttribute(batched_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem32) !=
-              cudaSuccess)
+      if (set_smem<0, 4>(kSmem64) || set_smem<0, 8>(kSmem64) || set_smem<1, 4>(kSmem32) || set_smem<1, 8>(kSmem32))
         return GBX_ERR_CUDA;
       g_attr = true;
     }
@@ -795,10 +840,24 @@ extern "C" int gbx_dposv_batched_ex(int batch, const int* n, const long long* of
   P.refine = refine;
   P.info = info;
   P.head = (unsigned long long*)work;
-  // default grid: every resident CTA slot; `ctas` overrides it
-  int grid = ctas > 0 ? ctas : (mode == 0 ? kCtas64 : kCtas32) * g_sms;
+  // All CTAs that are resident at once, `ctas` of them if given. As many as fit with eight warps have eight: then
+  // the systems are few, and what counts is one system's time (64 systems of order 100: FP64 296 us with four warps, 236 with
+  // eight, 128: 338 and 265, 1024: 60 ms and 51; 200 of 200 .. 900: 46 ms and 40, FP32 9.0 and 6.0); with more CTAs
+  // two small ones in the place of a large one do more (600 of order 64: 158 against 200 us).
+  int grid = std::min(ctas > 0 ? ctas : INT_MAX, ctas_per_sm(4) * g_sms);
   grid = std::max(1, std::min(grid, batch));
-  if (mode == 0) batched_kernel<0><<<grid, kThr, kSmem64, s>>>(P);
-  else batched_kernel<1><<<grid, kThr, kSmem32, s>>>(P);
+  P.sms = g_sms;
+  // When every system has a CTA at once, one CTA per SM takes them from the front of the order and the others from its
+  // end: largest first, an SM's other CTAs run small ones beside its large ones, and stop where the ends meet
+  // (FP64, all from the front before: 600 systems of 100 .. 400 13.8 -> 7.4 ms, of 20 .. 100 511 -> 344 us). With more
+  // systems the small ones are better kept for the end (4096 of 32 .. 512: FP64 62 against 55.7 ms, FP32 11.4 against 9.6).
+  P.front = batch <= ctas_per_sm(4) * g_sms ? std::min(grid, g_sms) : grid;
+  if (grid <= ctas_per_sm(8) * g_sms) {
+    if (mode == 0) batched_kernel<0, 8><<<grid, 256, kSmem64, s>>>(P);
+    else batched_kernel<1, 8><<<grid, 256, kSmem32, s>>>(P);
+  } else {
+    if (mode == 0) batched_kernel<0, 4><<<grid, 128, kSmem64, s>>>(P);
+    else batched_kernel<1, 4><<<grid, 128, kSmem32, s>>>(P);
+  }
   return cudaGetLastError() == cudaSuccess ? GBX_OK : GBX_ERR_CUDA;
 }
