@@ -4,7 +4,7 @@ tune_batched (small systems, gbx_dposv_batched_ex): for one batch (its size mix)
 candidate of
   * precision split: FP64, or FP32 factor + 1 or 2 FP64 refinement steps,
   * CTA schedule: queue order largest-first (longest processing time), natural, or
-    interleaved large/small; and the number of CTAs (1 or 2 per SM for FP32, 1 per SM for FP64),
+    interleaved large/small; and the number of CTAs (1, 2 or 4 per SM),
 keeps the candidates whose sampled backward error meets the tolerance, and returns the fastest.
 
 tune_mixed_batched (tiled systems, gbx_dposv_mixed_batched): times every tile size (256, 512),
@@ -14,7 +14,8 @@ each as the replay of a captured CUDA graph of the whole solve, keeps the candid
 every matrix met the tolerance, and returns the fastest. The tiles of the other tile sizes are
 made on the device by `retile`.
 
-Choices are cached per (GPU, size histogram, nrhs, tolerance) in a JSON file next to this module.
+Choices are cached per (GPU, size histogram, nrhs, tolerance) in a JSON file next to this module; those of
+tune_batched also per set of candidates and version of the kernel they were timed with.
 """
 import hashlib
 import json
@@ -23,6 +24,9 @@ import os
 import numpy as np
 
 _CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_autotune_cache.json")
+
+_KERNEL = 3  # of batched.cu: raised when what is best for a batch may have changed
+_CTAS_PER_SM = (1, 2, 4)  # of eight warps up to two, of four warps from there
 
 
 def _orders(sizes):
@@ -38,7 +42,7 @@ def _key(batch, tol):
     import torch
     hist = np.bincount(np.asarray(batch.sizes), minlength=1).tobytes()
     h = hashlib.sha1(hist).hexdigest()[:16]
-    return "%s|%s|%d|%g" % (torch.cuda.get_device_name(), h, batch.nrhs, tol)
+    return "%s|%s|%d|%g|v%d|%s" % (torch.cuda.get_device_name(), h, batch.nrhs, tol, _KERNEL, _CTAS_PER_SM)
 
 
 def _time(batch, mode, refine, ctas, reps):
@@ -91,7 +95,7 @@ def tune_batched(batch, rhs, tol=1e-14, reps=2, use_cache=True, sample_every=97)
     cands = []
     for mode, refine in (("fp64", 0), ("fp32", 1), ("fp32", 2)):
         for sched, order in orders.items():
-            for per_sm in (2, 4):  # four are resident (4096 systems, FP32: 13.8 ms with two, 9.0 with four)
+            for per_sm in _CTAS_PER_SM:
                 batch.set_order(order)
                 ms = _time(batch, mode, refine, per_sm * sms, reps)
                 be = _berr(batch, mats_fn, rhs, sample)
