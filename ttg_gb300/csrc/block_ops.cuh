@@ -181,21 +181,21 @@ __device__ __forceinline__ float rcp_nr(float d) {
 // 8 q + warp in x[h][q] (what lies above the diagonal is not read, and is garbage on return).
 // cb: 3 * 64 + 64 doubles, the last three columns of L, then the 64 pivot reciprocals;
 // *flag: 0 on entry (visible to all threads). Returns 0 or the 1-based index of the first bad pivot.
-template <bool kNamed, typename T>
-__device__ __forceinline__ int chol64_regs(T (&x)[2][8], int n, T* cb, int* flag) {
+template <bool kNamed>
+__device__ __forceinline__ int chol64_regs(double (&x)[2][8], int n, double* cb, int* flag) {
   const bool low = n > 32;  // rows 32.. exist
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto pivot = [&](auto qc, int j) {  // the warp that owns column j = 8 q + warp
     constexpr int q = decltype(qc)::value, h = q >> 2;
-    const T d = __shfl_sync(0xffffffffu, x[h][q], j & 31);
-    if (!(d > T(0))) {
+    const double d = __shfl_sync(0xffffffffu, x[h][q], j & 31);
+    if (!(d > 0.0)) {
       if (lane == 0) *flag = j + 1;
       return;
     }
-    T l, inv;
+    double l, inv;
     chol_pivot(d, l, inv);
     if (lane == 0) cb[192 + j] = inv;
-    T* b = cb + 64 * (j % 3);
+    double* b = cb + 64 * (j % 3);
     if (h == 0) {
       x[0][q] = lane == j ? l : x[0][q] * inv;
       b[lane] = x[0][q];
@@ -221,11 +221,11 @@ __device__ __forceinline__ int chol64_regs(T (&x)[2][8], int n, T* cb, int* flag
         stop = true;
         return;
       }
-      const T* b = cb + 64 * (j % 3);
-      const T l0 = b[lane], l1 = low ? b[lane + 32] : T(0);
+      const double* b = cb + 64 * (j % 3);
+      const double l0 = b[lane], l1 = low ? b[lane + 32] : 0.0;
       auto update = [&](auto q2c) {
         constexpr int q2 = decltype(q2c)::value;
-        const T lc = b[8 * q2 + warp];
+        const double lc = b[8 * q2 + warp];
         if (q2 < 4) x[0][q2] = fma(-l0, lc, x[0][q2]);
         if (low) x[1][q2] = fma(-l1, lc, x[1][q2]);
       };
@@ -243,12 +243,12 @@ __device__ __forceinline__ int chol64_regs(T (&x)[2][8], int n, T* cb, int* flag
         }
       } else {
         if (warp == jj && j > 0) {  // what this warp put off while it took pivot j
-          const T* bp = cb + 64 * ((j - 1) % 3);
-          const T m0 = bp[lane], m1 = low ? bp[lane + 32] : T(0);
+          const double* bp = cb + 64 * ((j - 1) % 3);
+          const double m0 = bp[lane], m1 = low ? bp[lane + 32] : 0.0;
 #pragma unroll
           for (int q2 = q + 1; q2 < 8; ++q2) {
             if (8 * q2 + warp < n) {
-              const T lc = bp[8 * q2 + warp];
+              const double lc = bp[8 * q2 + warp];
               if (q2 < 4) x[0][q2] = fma(-m0, lc, x[0][q2]);
               if (low) x[1][q2] = fma(-m1, lc, x[1][q2]);
             }
@@ -258,7 +258,7 @@ __device__ __forceinline__ int chol64_regs(T (&x)[2][8], int n, T* cb, int* flag
         for (int q2 = q; q2 < 8; ++q2) {
           const int c = 8 * q2 + warp;
           if (c > j && c < n) {
-            const T lc = b[c];
+            const double lc = b[c];
             if (q2 < 4) x[0][q2] = fma(-l0, lc, x[0][q2]);
             if (low) x[1][q2] = fma(-l1, lc, x[1][q2]);
           }
@@ -284,8 +284,8 @@ __device__ __forceinline__ int chol64_regs(T (&x)[2][8], int n, T* cb, int* flag
 // the diagonal, L(c, j) / L(j, j) at Ls[j ldl + c] (c > j), so that one FMA a column is on the serial chain; the
 // divisions of the results are taken at the end. rinv: the reciprocals of L's diagonal; both in shared memory
 // and visible; xb: 2 R G doubles.
-template <int R, int G, int NC, bool kNamed, typename T>
-__device__ __forceinline__ void trsm_regs(T (&x)[G][NC], int n, const T* Ls, int ldl, const T* rinv, T* xb) {
+template <int R, int G, int NC, bool kNamed>
+__device__ __forceinline__ void trsm_regs(double (&x)[G][NC], int n, const double* Ls, int ldl, const double* rinv, double* xb) {
   constexpr int P = 256 / R;  // columns dealt in one round
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = lane % R, col = (32 / R) * warp + lane / R;
@@ -299,13 +299,13 @@ __device__ __forceinline__ void trsm_regs(T (&x)[G][NC], int n, const T* Ls, int
     for (int jj = 0; jj < P; ++jj) {
       const int j = P * q + jj;
       if (j >= n) return;
-      T xj[G];
+      double xj[G];
 #pragma unroll
       for (int g = 0; g < G; ++g) xj[g] = xb[(j & 1) * R * G + g * R + r];
-      const T* Lj = Ls + (long long)j * ldl;
+      const double* Lj = Ls + (long long)j * ldl;
       auto publish = [&](auto q2c) {  // column j + 1: final after this update
         constexpr int q2 = decltype(q2c)::value;
-        const T l = Lj[j + 1];
+        const double l = Lj[j + 1];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
           x[g][q2] = fma(-xj[g], l, x[g][q2]);
@@ -323,7 +323,7 @@ __device__ __forceinline__ void trsm_regs(T (&x)[G][NC], int n, const T* Ls, int
       for (int q2 = q; q2 < NC; ++q2) {
         const int c = P * q2 + col;
         if (c > j + 1 && c < n) {
-          const T l = Lj[c];
+          const double l = Lj[c];
 #pragma unroll
           for (int g = 0; g < G; ++g) x[g][q2] = fma(-xj[g], l, x[g][q2]);
         }
@@ -343,7 +343,7 @@ __device__ __forceinline__ void trsm_regs(T (&x)[G][NC], int n, const T* Ls, int
 #pragma unroll
   for (int q = 0; q < NC; ++q)
     if (P * q + col < n) {
-      const T ri = rinv[P * q + col];
+      const double ri = rinv[P * q + col];
 #pragma unroll
       for (int g = 0; g < G; ++g) x[g][q] *= ri;
     }
@@ -557,15 +557,6 @@ __device__ __forceinline__ int op_potrf_f64(double* A, int lda, int n, double* s
   return info != 0 ? 64 + info : 0;
 }
 
-// ------------------------------------------------------------------------------------------------
-// block POTRF (lower, n <= 128): FP64 in registers (op_potrf_f64); FP32 in shared memory, blocked by
-// 32 columns:
-//   1. warp 0 factors the 32 x 32 diagonal block (warp-synchronous, no CTA barrier per column)
-//   2. every thread solves one row below the block against it (row-wise substitution)
-//   3. all threads apply the block's rank-32 update to the trailing lower triangle
-// Returns 0 or the 1-based local index of the first non-positive pivot (LAPACK info); the strict
-// upper triangle of A is not touched. smem: 128 * 128 elements + 1 int.
-// ------------------------------------------------------------------------------------------------
 // One row of a 32-column panel held in registers: x := x * L_blk^{-T} (row-wise forward
 // substitution against the panel's lower triangle Lp, column-major with leading dimension ldp).
 // rinv (optional): the 32 reciprocals of the panel's diagonal at rinv[rinv_at(c)], computed once
@@ -614,118 +605,6 @@ __device__ __forceinline__ void col_solve32(float (&x)[32], const float* Lp, int
     for (int r = c + 1; r < 32; ++r) x[r] = fmaf(-l[r], x[c], x[r]);
     if ((c + 1) % 8 == 0 && c < 31) __syncwarp();  // keeps the loads hoisted at most 8 columns ahead
   }
-}
-
-template <typename T, bool kNamed = false>
-__device__ int op_potrf(T* A, int lda, int n, T* sm) {
-  if constexpr (sizeof(T) == 8) return op_potrf_f64<kNamed>(A, lda, n, sm);
-  T* S = sm;                              // col-major, ld 128
-  int* flag = (int*)(sm + kBlk * kBlk);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) *flag = 0;
-  for (int idx = tid; idx < kBlk * n; idx += kThreads) {
-    const int i = idx & (kBlk - 1), j = idx >> 7;
-    if (i < n && i >= j) S[i + kBlk * j] = __ldcg(A + i + (long long)j * lda);
-  }
-  ops_sync<kNamed>();
-  int info = 0;
-  for (int p0 = 0; p0 < n; p0 += 32) {
-    const int pw = min(32, n - p0);
-    if (warp == 0) {
-      // 32 x 32 diagonal block: lane = row, the row in registers, columns exchanged by shuffles
-      T x[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) x[c] = (lane < pw && c <= lane) ? S[(p0 + lane) + kBlk * (p0 + c)] : T(0);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (j < pw) {
-          const T d = __shfl_sync(0xffffffffu, x[j], j);
-          if (!(d > T(0))) {  // same value in every lane: the whole warp leaves together
-            if (lane == 0) *flag = p0 + j + 1;
-            break;
-          }
-          T ljj, inv;
-          chol_pivot(d, ljj, inv);
-          if (lane == 0) S[p0 + rinv_at(j, kBlk) + kBlk * p0] = inv;  // for the rows below the block
-          // column j of L in every lane (0 above the diagonal); selects, not branches, so the
-          // warp never diverges inside the column loop
-          const T lij = lane == j ? ljj : (lane > j ? x[j] * inv : T(0));
-          x[j] = lij;
-#pragma unroll
-          for (int cc = j + 1; cc < 32; ++cc) {
-            const T lcj = __shfl_sync(0xffffffffu, lij, cc);
-            const T upd = fma(-lij, lcj, x[cc]);
-            x[cc] = lane >= cc ? upd : x[cc];
-          }
-        }
-      }
-      __syncwarp();
-      if (*flag == 0 && lane < pw)
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c <= lane) S[(p0 + lane) + kBlk * (p0 + c)] = x[c];
-    }
-    ops_sync<kNamed>();
-    info = *flag;
-    if (info) break;
-    // rows below the block: X := X L_d^{-T}, each thread one row in registers
-    const int rb = p0 + pw;
-    for (int r = rb + tid; r < n; r += kThreads) {
-      T x[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) x[c] = c < pw ? S[r + kBlk * (p0 + c)] : T(0);
-      row_solve32<T>(x, S + p0 + kBlk * p0, kBlk, pw, S + p0 + kBlk * p0);
-#pragma unroll
-      for (int c = 0; c < 32; ++c)
-        if (c < pw) S[r + kBlk * (p0 + c)] = x[c];
-    }
-    ops_sync<kNamed>();
-    // trailing update S(i, c) -= sum_k S(i, k) S(c, k), p0+pw <= c <= i < n
-    const int t0 = p0 + pw, t = n - t0;
-    if (t > 0) {  // 4 x 4 register blocks
-      const int nb4 = (t + 3) / 4;
-      const int nblk = nb4 * (nb4 + 1) / 2;
-      for (int q = tid; q < nblk; q += kThreads) {
-        int bj = 0, rem = q;  // lower 4 x 4 block (bi >= bj)
-        while (rem >= nb4 - bj) {
-          rem -= nb4 - bj;
-          ++bj;
-        }
-        const int bi = bj + rem;
-        const int i0 = t0 + 4 * bi, c0 = t0 + 4 * bj;
-        T acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = T(0);
-        for (int k = p0; k < p0 + pw; ++k) {
-          T vi[4], vc[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) vi[a] = (i0 + a < n) ? S[(i0 + a) + kBlk * k] : T(0);
-#pragma unroll
-          for (int b = 0; b < 4; ++b) vc[b] = (c0 + b < n) ? S[(c0 + b) + kBlk * k] : T(0);
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = fma(vi[a], vc[b], acc[a][b]);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int i = i0 + a, c = c0 + b;
-            if (i < n && c < n && i >= c) S[i + kBlk * c] -= acc[a][b];
-          }
-      }
-    }
-    ops_sync<kNamed>();
-  }
-  for (int idx = tid; idx < kBlk * n; idx += kThreads) {
-    const int i = idx & (kBlk - 1), j = idx >> 7;
-    if (i < n && i >= j) __stcg(A + i + (long long)j * lda, S[i + kBlk * j]);
-  }
-  ops_sync<kNamed>();
-  return info;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1148,84 +1027,6 @@ static __device__ __noinline__ void chain_gemm_f32(const float* A, int lda, cons
     }
   }
   __syncthreads();
-}
-
-// Triangular solves of one right-hand side held in shared memory xs[0..n) against the lower
-// factor L (column-major, ld), by 32-column panels: warp 0 solves the panel's triangle with its
-// rows in registers, the solved value broadcast by a shuffle and the diagonal's reciprocals taken
-// once per panel (an FP64 division is ~500 clocks of a warp on GB300), then the whole CTA applies
-// the panel to the other rows (two CTA barriers per panel instead of two per column).
-template <typename T>
-__device__ void fwd_solve(const T* L, int n, int ld, T* xs) {  // L y = x
-  __shared__ T tri[32 * 33];  // the panel's 32 x 32 triangle, staged once per panel
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int p0 = 0; p0 < n; p0 += 32) {
-    const int pw = min(32, n - p0);
-    for (int idx = tid; idx < 32 * 32; idx += blockDim.x) {
-      const int r = idx & 31, c = idx >> 5;
-      tri[r + 33 * c] = (r < pw && c < pw && r >= c) ? L[(p0 + r) + (long long)(p0 + c) * ld] : T(0);
-    }
-    __syncthreads();
-    if (warp == 0) {  // lane = row of the panel, x in a register; the reciprocals once per panel
-      T x = lane < pw ? xs[p0 + lane] : T(0);
-      const T ri = lane < pw ? T(1) / tri[lane * 34] : T(0);
-      for (int c = 0; c < pw; ++c) {
-        const T xc = __shfl_sync(0xffffffffu, x * ri, c);
-        if (lane == c) x = xc;
-        else if (lane > c) x = fma(-tri[lane + 33 * c], xc, x);
-      }
-      if (lane < pw) xs[p0 + lane] = x;
-    }
-    __syncthreads();
-    for (int i = p0 + pw + tid; i < n; i += blockDim.x) {
-      T s = T(0);
-#pragma unroll 8
-      for (int c = 0; c < pw; ++c) s += L[i + (long long)(p0 + c) * ld] * xs[p0 + c];
-      xs[i] -= s;
-    }
-    __syncthreads();
-  }
-}
-
-template <typename T>
-__device__ void bwd_solve(const T* L, int n, int ld, T* xs) {  // L^T x = y
-  __shared__ T tri[32 * 33];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int last = ((n - 1) / 32) * 32;
-  for (int p0 = last; p0 >= 0; p0 -= 32) {
-    const int pw = min(32, n - p0);
-    // contributions of the already solved rows below the panel: xs[r] -= sum_i L(i, r) x_i
-    for (int r = warp; r < pw; r += blockDim.x / 32) {
-      T s = T(0);
-      for (int i = p0 + pw + lane; i < n; i += 32) s += L[i + (long long)(p0 + r) * ld] * xs[i];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) xs[p0 + r] -= s;
-    }
-    for (int idx = tid; idx < 32 * 32; idx += blockDim.x) {
-      const int r = idx & 31, c = idx >> 5;
-      tri[r + 33 * c] = (r < pw && c < pw && r >= c) ? L[(p0 + r) + (long long)(p0 + c) * ld] : T(0);
-    }
-    __syncthreads();
-    if (warp == 0) {  // as in fwd_solve, from the last row up
-      T x = lane < pw ? xs[p0 + lane] : T(0);
-      const T ri = lane < pw ? T(1) / tri[lane * 34] : T(0);
-      for (int c = pw - 1; c >= 0; --c) {
-        const T xc = __shfl_sync(0xffffffffu, x * ri, c);
-        if (lane == c) x = xc;
-        else if (lane < c) x = fma(-tri[c + 33 * lane], xc, x);
-      }
-      if (lane < pw) xs[p0 + lane] = x;
-    }
-    __syncthreads();
-  }
-}
-
-// x := (L L^T)^{-1} x
-template <typename T>
-__device__ void solve_vec(const T* L, int n, int ld, T* xs) {
-  fwd_solve<T>(L, n, ld, xs);
-  bwd_solve<T>(L, n, ld, xs);
 }
 
 }  // namespace gbx

@@ -199,7 +199,7 @@ __device__ inline Mini mini_decode(int sub, int nb) {
 // SYRK updates: FP64 when the tile's condition estimate max_i a_ii / min_i a_ii (a lower bound of its
 // 2-norm condition number) exceeds P.fp64_cond, or when a diagonal entry is not positive; else FP32.
 // The FP64 route copies the tile's lower triangle into its FP64 scratch tile, runs the same
-// mini-flowgraph in FP64 there (op_potrf / op_trsm / op_gemm_nt<double>), and each block's final
+// mini-flowgraph in FP64 there (potrf_mini_fp64), and each block's final
 // writer (PF(j) for block (j,j), PT(j,i) for block (i,j)) also rounds the block into W.
 __device__ bool choose_fp64_route(const Params& P, const float* A, int n, float* sm) {
   float mn = 3.0e38f, mx = 0.f;

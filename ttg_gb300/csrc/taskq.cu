@@ -174,7 +174,7 @@ __device__ void potrf_tile(const Op& o, double* sm) {
   if (threadIdx.x == 0) s_bad = 0;
   __syncthreads();
   for (int p = 0; p < nb; ++p) {
-    const int info = op_potrf<double>(blk(p, p), ld, dim(p), sm);
+    const int info = op_potrf_f64<false>(blk(p, p), ld, dim(p), sm);
     if (threadIdx.x == 0) s_bad = info ? p * kBlk + info : 0;
     __syncthreads();
     if (s_bad) break;
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) taskq_kernel(RunParams P) {
   }
 }
 
-constexpr size_t kSmem = (size_t)kBlk * kBlk * sizeof(double) + 64;  // op_potrf<double>, the largest
+constexpr size_t kSmem = std::max({(size_t)kPotrf64Smem, op_trsm_smem_elems<double>(), (size_t)4 * kKC * kBlk}) * sizeof(double);
 
 }  // namespace taskq
 }  // namespace gbx
