@@ -628,6 +628,7 @@ struct Params {
   unsigned long long* head;  // matrices taken from the front of the order (low half) and its end (high half) after the first
   int front;                 // CTAs that take from the front
   int sms;
+  bool own;                  // a CTA's first matrix is given by its number
 };
 
 // R right-hand sides b (column-major, n x R) of one factorised matrix, in place
@@ -676,12 +677,13 @@ template <int MODE, int W>
 __global__ void __launch_bounds__(32 * W, ctas_per_sm(W)) batched_kernel(Params P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_idx;
-  // The first matrix is the CTA's own, so that it is known which ones share an SM (CTAs go to the SMs in turn, and they all
+  // The first matrix is the CTA's own (P.own), so that it is known which ones share an SM (CTAs go to the SMs in turn, and they all
   // start at about the same time): every second round of SMs in reverse, and from the end of the order the other way round
   // than from its front. Then what is left, from the CTA's end.
   const int wave = (int)blockIdx.x / P.sms, in_wave = min(P.sms, P.front - wave * P.sms), at = (int)blockIdx.x % P.sms;
   int first = (int)blockIdx.x >= P.front ? P.batch - 1 - ((int)blockIdx.x - P.front)
                                          : wave * P.sms + (wave & 1 ? in_wave - 1 - at : at);
+  if (!P.own) first = -1;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -689,7 +691,8 @@ __global__ void __launch_bounds__(32 * W, ctas_per_sm(W)) batched_kernel(Params 
       if (first < 0) {
         const bool front = (int)blockIdx.x < P.front;
         const unsigned long long h = atomicAdd(P.head, front ? 1ULL : 1ULL << 32);
-        const long long f = P.front + (long long)(h & 0xffffffffULL), e = gridDim.x - P.front + (long long)(h >> 32);
+        const long long f = (P.own ? P.front : 0) + (long long)(h & 0xffffffffULL);
+        const long long e = (P.own ? gridDim.x - P.front : 0) + (long long)(h >> 32);
         t = f + e >= P.batch ? -1 : front ? f : P.batch - 1 - e;  // (f and e of them are taken)
       }
       s_idx = t >= 0 ? P.order[t] : -1;
@@ -851,7 +854,11 @@ extern "C" int gbx_dposv_batched_ex(int batch, const int* n, const long long* of
   // end: largest first, an SM's other CTAs run small ones beside its large ones, and stop where the ends meet
   // (FP64, all from the front before: 600 systems of 100 .. 400 13.8 -> 7.4 ms, of 20 .. 100 511 -> 344 us). With more
   // systems the small ones are better kept for the end (4096 of 32 .. 512: FP64 62 against 55.7 ms, FP32 11.4 against 9.6).
-  P.front = batch <= ctas_per_sm(4) * g_sms ? std::min(grid, g_sms) : grid;
+  const bool one_round = batch <= ctas_per_sm(4) * g_sms;
+  P.front = one_round ? std::min(grid, g_sms) : grid;
+  // Many systems in FP32 are bound by latency, not by what an SM's systems add up to: the first comers take the largest
+  // (4096 systems 8.85 ms, 9.0 by number, FP64 59.3 and 55.7; 1300 of up to 64 rows 139 us, 150 by number).
+  P.own = one_round || mode == 0;
   if (grid <= ctas_per_sm(8) * g_sms) {
     if (mode == 0) batched_kernel<0, 8><<<grid, 256, kSmem64, s>>>(P);
     else batched_kernel<1, 8><<<grid, 256, kSmem32, s>>>(P);
