@@ -30,7 +30,7 @@ namespace batched {
 constexpr int kMaxN = 1024;  // largest matrix order of the batched kernel (shared-memory vectors)
 // One matrix keeps one CTA busy in spurts (a chain of pivots, a block product, a chain of panel solves), so
 // a CTA is small and four matrices share an SM; two with twice the warps when there are few (gbx_dposv_batched_ex).
-// 4096 matrices of 32 .. 512 rows: FP64 90.2 -> 55.7 ms with one CTA of 256 threads per SM before (the FP64 pipe alone
+// 4096 matrices of 32 .. 512 rows: FP64 90.2 -> 52.7 ms with one CTA of 256 threads per SM before (the FP64 pipe alone
 // needs 46), FP32 and two refinements 14.4 -> 8.9 (two CTAs of 256).
 constexpr int kPan = 64;            // largest block edge of the factorisation
 constexpr int kCk = 8;              // k-chunk of the block products
